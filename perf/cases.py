@@ -250,3 +250,64 @@ TOLERANCE = {
     # the reference's own roundings, bit for bit
     "dequantize": {"fp16": "exact", "bf16": "exact"},
 }
+
+
+# ---------------------------------------------------------------------------------------------
+# The same arithmetic in 64 bits, by torch alone
+# ---------------------------------------------------------------------------------------------
+def _expanded(w, k, case):
+    """(q - 8) * s - z (int4; int8 without the 8) of packed rows, in fp64."""
+    wq, s, z = w
+    if case["quant"] == "int4":
+        q = torch.empty((wq.shape[0], k), dtype=torch.float64, device=wq.device)
+        q[:, 0::2], q[:, 1::2] = (wq & 15).double() - 8.0, (wq >> 4).double() - 8.0
+    else:
+        q = wq.double()
+    g = min(case["group"], k)
+    q *= s.double().repeat_interleave(g, dim=1)[:, :k]
+    if z is not None:
+        q -= z.double().repeat_interleave(g, dim=1)[:, :k]
+    return q
+
+
+def _project(x, w, case):
+    """x @ W^T, expanded a block of rows at a time."""
+    k = x.shape[1]
+    rows = max(1, (1 << 27) // k)
+    parts = [x @ _expanded([None if t is None else t[i:i + rows] for t in w], k, case).t()
+             for i in range(0, w[0].shape[0], rows)]
+    return torch.cat(parts, dim=1)
+
+
+def _normed(x, r, w):
+    s = x.double() + r.double()
+    return s / torch.sqrt(s.pow(2).mean(dim=1, keepdim=True) + 1e-6) * w.double(), s
+
+
+def exact(case, seed):
+    """What ``run`` returns for these inputs, without any rounding between the operators."""
+    kind, k = case["kind"], case["k"]
+    if kind == "step":
+        gen = torch.Generator(device="cuda").manual_seed(seed)
+        dt, m, h = DTYPES[case["dtype"]], case["m"], case["h"]
+        x, r = _randn(gen, (m, k), dt), _randn(gen, (m, k), dt)
+        nw = (1.0 + 0.1 * torch.randn(k, generator=gen, device="cuda")).to(dt)
+        gu, down = _weights(gen, 2 * h, k, case), _weights(gen, k, h, case)
+        hid, res = _normed(x, r, nw)
+        both = _project(hid, gu, case)
+        act = torch.nn.functional.silu(both[:, :h]) * both[:, h:]
+        return {"y": _project(act, down, case) + res, "residual": res, "act": act}
+    st = prepare(case, seed)
+    if kind == "norm":
+        return _normed(st["x"], st["r"], st["w"])
+    if kind == "dequantize":
+        w = _expanded(st["w"], k, case)
+        return w.view(-1) if case["flat"] else w
+    y = _project(st["x"].cuda().double(), st["w"], case)
+    if kind == "host":
+        return y.cpu()
+    if st["bias"] is not None:
+        y = y + st["bias"].double()
+    if st["res"] is not None:
+        y = y + st["res"].double()
+    return torch.nn.functional.silu(y) if case["epilogue"] == "bias_silu" else y
