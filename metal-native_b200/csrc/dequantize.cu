@@ -8,9 +8,9 @@
 //  * dequantize_flat_kernel: the reference's dequantize_int{4,8}_to_fp16 kernels
 //    (shaders/dequantize_kernel.metal): scale only, flat group index.
 //
-// Both are pure streaming: 0.5-1 byte read and 2-4 bytes written per weight, so the
-// bound is HBM write bandwidth.  Each thread converts 8 consecutive weights of one
-// row (one 32-bit word of nibbles, or 8 bytes) and writes them with 16/32-byte stores.
+// Both are pure streaming: 0.5-1 byte read and 2-4 bytes written per weight, so the bound is HBM,
+// writes above all.  One kernel serves both (dequantize_vec8_kernel) wherever eight consecutive
+// weights share a group and are aligned; the one-thread-per-element kernels take the rest.
 #include "mnq_common.cuh"
 
 namespace mnq {
@@ -37,46 +37,96 @@ __device__ __forceinline__ float dequant_value(int q_centred, float s, float z)
 
 template <typename OutT, int N> struct alignas(sizeof(OutT) * N) Pack { OutT v[N]; };
 
-// One thread = 8 consecutive k of one row.  Requires K % 8 == 0.
-template <int QUANT, typename OutT>
-__global__ void __launch_bounds__(256)
-dequantize_matrix_vec8_kernel(const uint8_t* __restrict__ wq, const void* __restrict__ scales,
-                              const void* __restrict__ zeros, OutT* __restrict__ out, int64_t N,
-                              int64_t K, int32_t group_size, int32_t G, int32_t scale_dtype)
-{
-    const int64_t k8_per_row = K >> 3;
-    const int64_t total = N * k8_per_row;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t n = i / k8_per_row;
-        const int64_t k0 = (i - n * k8_per_row) << 3;
-        int q[8];
-        if (QUANT == MNQ_INT4) {
-            const uint32_t w = ldg_stream_4(wq + n * (K >> 1) + (k0 >> 1));
-#pragma unroll
-            for (int e = 0; e < 8; ++e) q[e] = static_cast<int>((w >> (4 * e)) & 0xF) - 8;
-        } else {
-            const uint2 w = ldg_stream_8(wq + n * K + k0);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                q[e] = static_cast<int>(static_cast<int8_t>((w.x >> (8 * e)) & 0xFF));
-                q[e + 4] = static_cast<int>(static_cast<int8_t>((w.y >> (8 * e)) & 0xFF));
-            }
+// Division of indices below 2^31 by a value known at launch: one high multiplication and a shift.
+struct FastDiv {
+    uint32_t mul = 0, shift = 0;   // mul 0: division by one
+    static FastDiv by(uint32_t d)
+    {
+        FastDiv f;
+        if (d > 1) {
+            uint32_t l = 1;
+            while ((1ull << l) < d) ++l;
+            f.mul = static_cast<uint32_t>(((1ull << (31 + l)) + d - 1) / d);
+            f.shift = l - 1;
         }
+        return f;
+    }
+    __device__ __forceinline__ uint32_t operator()(uint32_t n) const { return mul ? __umulhi(n, mul) >> shift : n; }
+};
+
+// q of eight consecutive weights, as fp32.  A nibble (or byte + 128) in the low mantissa bits of 2^23 is
+// 2^23 + q exactly; the subtraction that centres it is exact.  (An integer conversion runs at a quarter of
+// the rate of these.)
+template <int QUANT> struct Ints8;
+template <> struct Ints8<MNQ_INT4> {
+    using Word = uint32_t;
+    static __device__ __forceinline__ Word load(const uint8_t* base, uint32_t i) { return ldg_stream_4(base + (size_t)i * 4); }
+    static __device__ __forceinline__ void run(Word w, float (&q)[8])
+    {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) q[e] = __uint_as_float(lop3<0xEA>(w >> (4 * e), 0xFu, 0x4B000000u)) - 8388616.f;
+    }
+};
+template <> struct Ints8<MNQ_INT8> {
+    using Word = uint2;
+    static __device__ __forceinline__ Word load(const uint8_t* base, uint32_t i) { return ldg_stream_8(base + (size_t)i * 8); }
+    static __device__ __forceinline__ void run(Word w, float (&q)[8])
+    {
+        const uint32_t u[2] = {w.x ^ 0x80808080u, w.y ^ 0x80808080u};
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+            q[e] = __uint_as_float(prmt(u[e >> 2], 0x4B000000u, 0x7440u + (e & 3))) - 8388736.f;
+    }
+};
+
+// Eight consecutive weights are a block; thread t of a CTA takes blocks t, t + 256, ... of the CTA's kUnroll * 256,
+// so every load and store instruction of a warp covers one contiguous run, and all loads of a thread are issued
+// before the first is used.  A block lies in one group (group size and row length are multiples of eight).  With
+// whole groups in every row the group of block i is i / (group / 8) over the whole matrix; rows that end in a
+// shorter group need the row first.
+// Bound by HBM.  [18944, 3584] int4, groups of 128, to fp16 (37 MB read, 136 MB written): 129 us with 64-bit
+// divisions per block, a division by the group size per weight and integer conversions; 33 us = 5.2 TB/s now
+// (two and eight blocks per thread: 36 and 41).
+constexpr int kUnroll = 4;
+template <int QUANT, typename OutT, bool HAS_Z>
+__global__ void __launch_bounds__(256)
+dequantize_vec8_kernel(const uint8_t* __restrict__ in, const void* __restrict__ scales, const void* __restrict__ zeros,
+                       OutT* __restrict__ out, uint32_t blocks, FastDiv per_row, uint32_t row_blocks, FastDiv per_group,
+                       uint32_t row_groups, int32_t scale_dtype)
+{
+    const uint32_t i0 = blockIdx.x * (256u * kUnroll) + threadIdx.x;
+    typename Ints8<QUANT>::Word w[kUnroll];
+    float s[kUnroll], z[kUnroll];
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u)
+        if (i0 + u * 256u < blocks) w[u] = Ints8<QUANT>::load(in, i0 + u * 256u);
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u) {
+        const uint32_t i = i0 + u * 256u;
+        if (i >= blocks) break;
+        uint32_t g;
+        if (row_groups) {
+            const uint32_t n = per_row(i);
+            g = n * row_groups + per_group(i - n * row_blocks);
+        } else {
+            g = per_group(i);
+        }
+        s[u] = widen16(scales, g, scale_dtype);
+        z[u] = HAS_Z ? widen16(zeros, g, scale_dtype) : 0.f;
+    }
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u) {
+        const uint32_t i = i0 + u * 256u;
+        if (i >= blocks) break;
+        float q[8];
+        Ints8<QUANT>::run(w[u], q);
         Pack<OutT, 8> o;
-        int g_prev = -1;
-        float s = 0.f, z = 0.f;
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-            const int g = static_cast<int>((k0 + e) / group_size);
-            if (g != g_prev) {
-                s = widen16(scales, n * G + g, scale_dtype);
-                z = zeros ? widen16(zeros, n * G + g, scale_dtype) : 0.f;
-                g_prev = g;
-            }
-            o.v[e] = OutCvt<OutT>::cvt(dequant_value(q[e], s, z));
+            const float p = __fmul_rn(q[e], s[u]);   // product and subtraction each rounded once, as in dequant_value
+            o.v[e] = OutCvt<OutT>::cvt(HAS_Z ? __fsub_rn(p, z[u]) : p);
         }
-        *reinterpret_cast<Pack<OutT, 8>*>(out + n * K + k0) = o;
+        *reinterpret_cast<Pack<OutT, 8>*>(out + (size_t)i * 8) = o;
     }
 }
 
@@ -108,67 +158,23 @@ dequantize_matrix_scalar_kernel(const uint8_t* __restrict__ wq, const void* __re
 }
 
 // Reference semantics of shaders/dequantize_kernel.metal: out[i] = half(q) * s[i / g]
-// in half arithmetic == RN_fp16 of the exact (fp32-representable) product.
+// in half arithmetic == RN_fp16 of the exact (fp32-representable) product.  One thread per element, from element
+// `first` on: unaligned buffers, group sizes that are no multiple of eight, and what is left of a last block.
 template <int QUANT>
 __global__ void __launch_bounds__(256)
-dequantize_flat_kernel(const uint8_t* __restrict__ in, const __half* __restrict__ scales,
-                       __half* __restrict__ out, int64_t num_elements, int32_t group_size, bool vec_ok)
+dequantize_flat_scalar_kernel(const uint8_t* __restrict__ in, const __half* __restrict__ scales,
+                              __half* __restrict__ out, int64_t first, int64_t num_elements, int32_t group_size)
 {
-    const int64_t n8 = (num_elements + 7) >> 3;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n8;
+    for (int64_t i = first + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < num_elements;
          i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t e0 = i << 3;
-        const bool full = vec_ok && (e0 + 8 <= num_elements);
-        int q[8];
-        if (full) {
-            if (QUANT == MNQ_INT4) {
-                const uint32_t w = ldg_stream_4(in + (e0 >> 1));
-#pragma unroll
-                for (int e = 0; e < 8; ++e) q[e] = static_cast<int>((w >> (4 * e)) & 0xF) - 8;
-            } else {
-                const uint2 w = ldg_stream_8(in + e0);
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    q[e] = static_cast<int>(static_cast<int8_t>((w.x >> (8 * e)) & 0xFF));
-                    q[e + 4] = static_cast<int>(static_cast<int8_t>((w.y >> (8 * e)) & 0xFF));
-                }
-            }
+        int q;
+        if (QUANT == MNQ_INT4) {
+            const uint8_t b = in[i >> 1];
+            q = static_cast<int>((i & 1) ? (b >> 4) : (b & 0xF)) - 8;
         } else {
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                const int64_t idx = e0 + e;
-                q[e] = 0;
-                if (idx < num_elements) {
-                    if (QUANT == MNQ_INT4) {
-                        const uint8_t b = in[idx >> 1];
-                        q[e] = static_cast<int>((idx & 1) ? (b >> 4) : (b & 0xF)) - 8;
-                    } else {
-                        q[e] = static_cast<int>(static_cast<int8_t>(in[idx]));
-                    }
-                }
-            }
+            q = static_cast<int>(static_cast<int8_t>(in[i]));
         }
-        Pack<__half, 8> o;
-        int64_t g_prev = -1;
-        float s = 0.f;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            const int64_t idx = e0 + e;
-            if (idx < num_elements) {
-                const int64_t g = idx / group_size;
-                if (g != g_prev) { s = __half2float(__ldg(scales + g)); g_prev = g; }
-                o.v[e] = __float2half_rn(__fmul_rn(static_cast<float>(q[e]), s));
-            } else {
-                o.v[e] = __ushort_as_half(0);
-            }
-        }
-        if (full) {
-            *reinterpret_cast<Pack<__half, 8>*>(out + e0) = o;
-        } else {
-#pragma unroll
-            for (int e = 0; e < 8; ++e)
-                if (e0 + e < num_elements) out[e0 + e] = o.v[e];
-        }
+        out[i] = __float2half_rn(__fmul_rn(static_cast<float>(q), __half2float(__ldg(scales + i / group_size))));
     }
 }
 
@@ -179,23 +185,79 @@ inline int grid_for(int64_t work_items, int sm_count)
     return static_cast<int>(blocks < 1 ? 1 : (blocks > cap ? cap : blocks));
 }
 
+// [rows, K] weights, K and the group size multiples of eight (or one group per row), aligned buffers.  Indices
+// are 32 bits wide in the kernel, so a matrix of more than 2^30 blocks goes in slices of whole rows.
+template <int QUANT, typename OutT>
+int launch_vec8(const uint8_t* in, const uint16_t* scales, const uint16_t* zeros, OutT* out, int64_t rows, int64_t K,
+                int64_t group_size, int32_t scale_dtype, cudaStream_t stream)
+{
+    const int64_t row_blocks = K / 8;
+    const int64_t g = group_size < K ? group_size : K;
+    const int64_t G = (K + g - 1) / g;
+    const bool whole = K % g == 0;
+    int64_t slice = (int64_t(1) << 30) / row_blocks;
+    if (slice < 1) return fail(MNQ_INVALID_ARGUMENT, "dequantize: rows of more than 2^33 weights are not supported");
+    for (int64_t n = 0; n < rows; n += slice) {
+        const int64_t here = rows - n < slice ? rows - n : slice;
+        const uint32_t blocks = static_cast<uint32_t>(here * row_blocks);
+        const unsigned grid = (blocks + 256u * kUnroll - 1) / (256u * kUnroll);
+        const uint8_t* at = in + n * (QUANT == MNQ_INT4 ? K / 2 : K);
+        auto* kern = zeros ? &dequantize_vec8_kernel<QUANT, OutT, true> : &dequantize_vec8_kernel<QUANT, OutT, false>;
+        kern<<<grid, 256, 0, stream>>>(at, scales + n * G, zeros ? zeros + n * G : nullptr, out + n * K, blocks,
+                                       FastDiv::by(static_cast<uint32_t>(row_blocks)), static_cast<uint32_t>(row_blocks),
+                                       FastDiv::by(static_cast<uint32_t>(g / 8)), whole ? 0u : static_cast<uint32_t>(G), scale_dtype);
+        const int rc = check_cuda(cudaGetLastError(), "dequantize launch");
+        if (rc) return rc;
+    }
+    return MNQ_SUCCESS;
+}
+
 template <int QUANT, typename OutT>
 int launch_matrix(const void* wq, const void* scales, const void* zeros, void* out, int64_t N,
                   int64_t K, int32_t group_size, int32_t G, int32_t scale_dtype, int sm_count,
                   cudaStream_t stream)
 {
-    const bool aligned = (reinterpret_cast<uintptr_t>(wq) % 8 == 0) &&
+    const bool aligned = (reinterpret_cast<uintptr_t>(wq) % (QUANT == MNQ_INT4 ? 4 : 8) == 0) &&
                          (reinterpret_cast<uintptr_t>(out) % (8 * sizeof(OutT)) == 0);
-    if (K % 8 == 0 && aligned) {
-        dequantize_matrix_vec8_kernel<QUANT, OutT><<<grid_for(N * (K / 8), sm_count), 256, 0, stream>>>(
-            static_cast<const uint8_t*>(wq), scales, zeros, static_cast<OutT*>(out), N, K, group_size,
-            G, scale_dtype);
-    } else {
-        dequantize_matrix_scalar_kernel<QUANT, OutT><<<grid_for(N * K, sm_count), 256, 0, stream>>>(
-            static_cast<const uint8_t*>(wq), scales, zeros, static_cast<OutT*>(out), N, K, group_size,
-            G, scale_dtype);
-    }
+    if (K % 8 == 0 && (group_size % 8 == 0 || group_size >= K) && aligned && K < (int64_t(1) << 33))
+        return launch_vec8<QUANT, OutT>(static_cast<const uint8_t*>(wq), static_cast<const uint16_t*>(scales),
+                                        static_cast<const uint16_t*>(zeros), static_cast<OutT*>(out), N, K, group_size,
+                                        scale_dtype, stream);
+    dequantize_matrix_scalar_kernel<QUANT, OutT><<<grid_for(N * K, sm_count), 256, 0, stream>>>(
+        static_cast<const uint8_t*>(wq), scales, zeros, static_cast<OutT*>(out), N, K, group_size,
+        G, scale_dtype);
     return check_cuda(cudaGetLastError(), "dequantize launch");
+}
+
+// A flat run of weights is a matrix whose rows are whole groups; what is left after the last whole group (and in
+// it, after the last block of eight) goes through the element kernel.
+template <int QUANT>
+int launch_flat(const uint8_t* in, const __half* scales, __half* out, int64_t num_elements, int32_t group_size,
+                int sm_count, cudaStream_t stream)
+{
+    const bool aligned = (reinterpret_cast<uintptr_t>(in) % (QUANT == MNQ_INT4 ? 4 : 8) == 0) &&
+                         (reinterpret_cast<uintptr_t>(out) % 16 == 0);
+    int64_t done = 0;
+    if (aligned && group_size % 8 == 0) {
+        const uint16_t* s16 = reinterpret_cast<const uint16_t*>(scales);
+        const int64_t groups = num_elements / group_size;
+        if (groups > 0) {
+            const int rc = launch_vec8<QUANT, __half>(in, s16, nullptr, out, groups, group_size, group_size, MNQ_FP16, stream);
+            if (rc) return rc;
+            done = groups * group_size;
+        }
+        const int64_t rest = (num_elements - done) / 8 * 8;   // of a last, shorter group: one row of its own
+        if (rest > 0) {
+            const int64_t bytes = QUANT == MNQ_INT4 ? done / 2 : done;
+            const int rc = launch_vec8<QUANT, __half>(in + bytes, s16 + groups, nullptr, out + done, 1, rest, rest, MNQ_FP16, stream);
+            if (rc) return rc;
+            done += rest;
+        }
+    }
+    if (done == num_elements) return MNQ_SUCCESS;
+    dequantize_flat_scalar_kernel<QUANT><<<grid_for(num_elements - done, sm_count), 256, 0, stream>>>(
+        in, scales, out, done, num_elements, group_size);
+    return check_cuda(cudaGetLastError(), "dequantize_flat launch");
 }
 
 }  // namespace
@@ -220,18 +282,11 @@ int launch_dequantize_matrix(const void* wq, const void* scales, const void* zer
 int launch_dequantize_flat(const void* in, const void* scales, void* out, int64_t num_elements,
                            int32_t group_size, int32_t quant, int sm_count, cudaStream_t stream)
 {
-    const bool vec_ok = (reinterpret_cast<uintptr_t>(in) % 8 == 0) &&
-                        (reinterpret_cast<uintptr_t>(out) % 16 == 0);
-    const int grid = grid_for((num_elements + 7) / 8, sm_count);
     if (quant == MNQ_INT4)
-        dequantize_flat_kernel<MNQ_INT4><<<grid, 256, 0, stream>>>(
-            static_cast<const uint8_t*>(in), static_cast<const __half*>(scales),
-            static_cast<__half*>(out), num_elements, group_size, vec_ok);
-    else
-        dequantize_flat_kernel<MNQ_INT8><<<grid, 256, 0, stream>>>(
-            static_cast<const uint8_t*>(in), static_cast<const __half*>(scales),
-            static_cast<__half*>(out), num_elements, group_size, vec_ok);
-    return check_cuda(cudaGetLastError(), "dequantize_flat launch");
+        return launch_flat<MNQ_INT4>(static_cast<const uint8_t*>(in), static_cast<const __half*>(scales),
+                                     static_cast<__half*>(out), num_elements, group_size, sm_count, stream);
+    return launch_flat<MNQ_INT8>(static_cast<const uint8_t*>(in), static_cast<const __half*>(scales),
+                                 static_cast<__half*>(out), num_elements, group_size, sm_count, stream);
 }
 
 }  // namespace mnq

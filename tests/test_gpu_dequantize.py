@@ -1,0 +1,48 @@
+"""The standalone dequantisation kernels at the edges of their dispatch, against the oracle, bit for bit."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import check as H
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def mn():
+    import metal_native
+    assert torch.cuda.is_available()
+    return metal_native
+
+
+# blocks of eight, 1024 blocks per CTA: one block, one CTA less a block, one CTA and one block; whole and shorter last
+# groups; group sizes that are no multiple of eight, one group per row, rows that are no multiple of eight
+@pytest.mark.parametrize("quant,N,K,g,zeros,sdt", [
+    ("int4", 1, 8, 8, True, torch.float16), ("int8", 1, 8, 32, False, torch.bfloat16),
+    ("int4", 1023, 8, 8, True, torch.bfloat16), ("int8", 41, 200, 40, True, torch.float16),
+    ("int4", 41, 200, 128, True, torch.float16), ("int8", 33, 4000, 96, False, torch.float16),
+    ("int4", 130, 1000, 1024, True, torch.bfloat16), ("int4", 9, 200, 20, True, torch.float16),
+    ("int8", 9, 203, 32, True, torch.float16),
+])
+def test_matrix(mn, quant, N, K, g, zeros, sdt):
+    import mnq_workloads as workloads
+    L = workloads.make_layer("t", 1, K, N, quant_type=quant, group_size=g, scale_dtype=sdt, asymmetric=zeros, seed=3)
+    ref = H.oracle_dequant(L)
+    d = L.to("cuda")
+    for dt in (torch.float32, torch.float16, torch.bfloat16):
+        got = mn.dequantize(d.wq, d.scales, d.zeros, g, quant, dt).cpu()
+        assert torch.equal(got, torch.from_numpy(ref).to(dt)), dt
+
+
+@pytest.mark.parametrize("quant,n,g,shift", [
+    ("int4", 8192, 32, 0), ("int4", 8192 + 8 + 6, 32, 0), ("int4", 14, 64, 0), ("int8", 1000, 24, 0), ("int8", 1003, 64, 0),
+    ("int4", 4096, 20, 0), ("int8", 4096, 64, 3), ("int4", 4096, 64, 2)])
+def test_flat(mn, quant, n, g, shift):
+    gen = torch.Generator().manual_seed(7)
+    nbytes = (n + 1) // 2 if quant == "int4" else n
+    q = torch.randint(0, 256, (nbytes + shift,), generator=gen, dtype=torch.uint8)
+    s = (torch.rand((n + g - 1) // g, generator=gen) * 0.02 + 0.001).to(torch.float16)
+    ref = oracle.dequantize_flat(q[shift:].numpy(), s.view(torch.int16).numpy().view(np.uint16), n, g, quant)
+    got = mn.dequantize_flat(q.cuda()[shift:], s.cuda(), g, quant, n).cpu()
+    assert np.array_equal(got.view(torch.int16).numpy().view(np.uint16), ref)
