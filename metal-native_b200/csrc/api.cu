@@ -236,12 +236,16 @@ int64_t gemv_max_m_for(int64_t K, int32_t group_size, int32_t quant, int32_t act
 
 // Decode kernels up to the threshold, the tensor-core kernel above it, the any-shape kernel for
 // whatever neither takes.
+constexpr int64_t kAnyShapeProducts = 4 << 20;
 int choose_path(const MatmulArgs& a)
 {
     int64_t gemv_max_m = gemv_max_m_for(a.K, a.group_size, a.quant, a.act_dtype);
-    // small layers of few rows: the tensor-core kernel from 17 tokens (not where it needs two bf16 tiles per k-block)
-    if (option_value(MNQ_OPT_GEMV_MAX_M) == 0 && gemv_max_m > 16 && few_rows_small_layer(a) &&
-        !(a.act_dtype == MNQ_BF16 && (a.group_size < a.K || a.zeros != nullptr)))
+    // small layers of few rows: the tensor-core kernel from 17 tokens (not where it needs two tiles per k-block, unless the
+    // decode kernel would be the register-prefetch one: 4128 x 4096 int4 fp16 at 32 tokens, groups of 32: 27.6 against
+    // 57.0 us; one group per row, which the streaming kernel takes: 24.4 against 18.0)
+    const bool two_tiles = a.act_dtype == MNQ_BF16 ? a.group_size < a.K || a.zeros != nullptr
+                                                   : odd_halves(a.K, a.group_size) && gemv_stream_supported(a, nullptr);
+    if (option_value(MNQ_OPT_GEMV_MAX_M) == 0 && gemv_max_m > 16 && few_rows_small_layer(a) && !two_tiles)
         gemv_max_m = 16;
     if (a.M <= gemv_max_m && gemv_supported(a)) return MNQ_PATH_GEMV;
     // 33 to 64 tokens of bf16 activations where the tensor-core kernel would need two bf16 tiles per
@@ -251,7 +255,11 @@ int choose_path(const MatmulArgs& a)
     if (a.M > 32 && a.M <= 64 && a.act_dtype == MNQ_BF16 && option_value(MNQ_OPT_GEMV_MAX_M) == 0 &&
         option_value(MNQ_OPT_BF16_FP16_TILES) == 0 && a.group_size < a.K && gemv_supported(a))
         return MNQ_PATH_GEMV;
-    if (a.M > gemv_max_m && gemm_supported(a)) return MNQ_PATH_GEMM;
+    // (a problem of a few million products with groups or rows of an odd number of 32s is over in the any-shape kernel
+    // before the tensor-core kernel has set up: 1.3 million (K, N, M = 160, 256, 33) 4.5 us, 7.3 million 11.0 against 6.8,
+    // 4.2 billion 3570 against 52)
+    if (a.M > gemv_max_m && gemm_supported(a) && !(odd_halves(a.K, a.group_size) && a.M * a.N * a.K < kAnyShapeProducts))
+        return MNQ_PATH_GEMM;
     if (a.M <= 32 && gemv_supported(a)) return MNQ_PATH_GEMV;   // e.g. K not a multiple of 64
     return MNQ_PATH_GENERIC;
 }

@@ -67,6 +67,8 @@ struct GemmParams {
     const void* zeros;
     void* out;
     int M, N, K;
+    int kb_total;       // 64-k blocks, the last one half empty where K is an odd multiple of 32
+    int half_blocks;    // 1: the two 32-k halves of a k-block may differ in group (groups of an odd number of 32s) or the last half lies past K
     long long ldc;
     int row_bytes;
     int group_size;     // >= K: one group
@@ -371,6 +373,12 @@ struct BSplit {};
 // fp16's 11 significant bits, as with fp16 activations (noise of about 2.8e-4 of the output RMS), where the
 // two-tile path keeps 16.
 struct HalfTile {};
+// fp16 activations with groups, or rows, of an odd number of 32s: as BSplit with fp16 values.  (Multiples of 64 take one
+// fp16 tile.  These shapes came from the any-shape kernel, which keeps weights in fp32, and two tiles keep its
+// accuracy: the weight, computed in fp32 from scale and zero divided by the row's 2^E as for HalfTile, is
+// RN(w) + RN(w - RN(w)), within 2^-25 of the row's largest; measured against fp64 the results of both are the same
+// 2.1e-4, the rounding of the output.)
+struct HSplit {};
 
 template <int QUANT> struct SplitChunk;
 template <> struct SplitChunk<MNQ_INT4> {
@@ -402,7 +410,7 @@ template <> struct SplitChunk<MNQ_INT8> {
         }
     }
 };
-template <int QUANT>
+template <int QUANT, bool HALF>
 __device__ __forceinline__ void split_chunk(const uint32_t* w, float s, float nz, uint4& hi, uint4& lo)
 {
     float q[8];
@@ -411,6 +419,13 @@ __device__ __forceinline__ void split_chunk(const uint32_t* w, float s, float nz
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const float a = fmaf(q[2 * i], s, nz), b = fmaf(q[2 * i + 1], s, nz);
+        if (HALF) {
+            const __half2 h = __floats2half2_rn(a, b);
+            const float2 back = __half22float2(h);
+            H[i] = h2_as_u32(h);
+            L[i] = h2_as_u32(__floats2half2_rn(a - back.x, b - back.y));
+            continue;
+        }
         const __nv_bfloat162 h2 = __floats2bfloat162_rn(a, b);
         H[i] = b2_as_u32(h2);
         const float ra = a - __uint_as_float(H[i] << 16), rb = b - __uint_as_float(H[i] & 0xFFFF0000u);
@@ -551,7 +566,8 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap
     constexpr int KPR = 128 / KB_BYTES;                 // k-blocks covered by one raw stage (128 packed bytes per row)
     constexpr int RAW_BYTES = BN * 128;
     constexpr bool IS_BF16 = std::is_same<T, __nv_bfloat16>::value;
-    constexpr bool SPLIT = std::is_same<TT, BSplit>::value;
+    constexpr bool HSPLIT = std::is_same<TT, HSplit>::value;
+    constexpr bool SPLIT = std::is_same<TT, BSplit>::value || HSPLIT;   // two tiles per k-block
     constexpr bool RAW = std::is_same<TT, RawInt>::value;      // fp16 tiles of raw integers, fp16 activations whatever T is
     constexpr bool HALF_T = std::is_same<TT, HalfTile>::value; // fp16 tiles and fp16 copies of bf16 activations
     constexpr bool MMA_BF16 = IS_BF16 && !RAW && !HALF_T;
@@ -562,7 +578,7 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap
 
     extern __shared__ unsigned char smem_raw[];
     __shared__ uint32_t tmem_base_slot;
-    __shared__ float row_up[HALF_T ? BN : 1];   // HalfTile: 2^E of every weight row of the tile
+    __shared__ float row_up[HALF_T || HSPLIT ? BN : 1];   // HalfTile, HSplit: 2^E of every weight row of the tile
     // ready[8], done[8], accum, raw_full[4], raw_empty[4]
     __shared__ __align__(8) unsigned long long bars[2 * 8 + 1 + 2 * 4];
 
@@ -582,7 +598,7 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap
     const int n0 = tile_x * BN;
     const int m0 = blockIdx.y * p.tok;
     const int kb_begin = part * kb_per_part;
-    const int num_kb = min(p.K / BK, kb_begin + kb_per_part) - kb_begin;   // k-blocks of this part
+    const int num_kb = min(p.kb_total, kb_begin + kb_per_part) - kb_begin;   // k-blocks of this part
     // Rings: S weight tiles, SB activation stages (one stage = the nh tiles of one k-block).
     // Synchronisation is per k-block, on D = max(S, SB) barrier pairs indexed kb % D:
     // ready[kb % D] completes when the k-block's weight tile is dequantised (one arrival per
@@ -752,15 +768,15 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap
         uint32_t xoff[8];
 #pragma unroll
         for (int c = 0; c < 8; ++c) xoff[c] = (uint32_t)((c ^ (row & 7)) << 4);
-        // k-blocks per quantisation group as a shift when it is a power of two (it almost always is)
-        const int kbg = (p.group_size >= p.K) ? 1 : p.group_size / BK;
-        const int kbg_shift = (kbg & (kbg - 1)) == 0 ? 31 - __clz(kbg) : -1;
+        // half k-blocks per quantisation group as a shift when it is a power of two (it almost always is)
+        const int hpg = (p.group_size >= p.K) ? 1 : p.group_size / (BK / 2);
+        const int hpg_shift = (hpg & (hpg - 1)) == 0 ? 31 - __clz(hpg) : -1;
         const bool one_group = p.group_size >= p.K;
         const int g_first = one_group ? 0 : (kb_begin * BK) / p.group_size;
         if (!RAW) {   // scale | zero << 16 of every (row, group) this CTA touches, [group][row]
             const unsigned short* sc16 = static_cast<const unsigned short*>(p.scales);
             const unsigned short* zr16 = static_cast<const unsigned short*>(p.zeros);
-            const int g_last = one_group ? 0 : ((kb_begin + num_kb) * BK - 1) / p.group_size;
+            const int g_last = one_group ? 0 : min(((kb_begin + num_kb) * BK - 1) / p.group_size, p.G - 1);
             const int gc = g_last - g_first + 1;          // <= p.table_groups
             // eight entries per thread and pass, all loads issued before the first store: the whole
             // table costs one or two global round trips instead of one per entry
@@ -775,7 +791,7 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap
             const size_t rowsrc = (size_t)min(n0 + rr, p.N - 1) * p.G + g_first;
             const unsigned short* zsrc = zr16 ? zr16 : sc16;
             float down = 1.f;   // HalfTile: 2^-E of this row
-            if (HALF_T) {
+            if (HALF_T || HSPLIT) {
                 // largest of 8 |s| and |z| over the row's groups of this split (both threads of the row)
                 const bool sbf = p.scale_dtype == MNQ_BF16;
                 auto mag = [&](uint32_t bits) {
@@ -827,6 +843,7 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap
             asm volatile("bar.sync 1, 256;" ::: "memory");   // the eight dequantise warps only
         }
 
+        const float row_down = HSPLIT ? __uint_as_float((254u << 23) - __float_as_uint(row_up[row])) : 1.f;   // 1 / 2^E
         const uint32_t ready_at = PAIR ? map_to_rank(ready0, 0) : ready0;   // the leader's barriers
         // This warp takes every other k-block of the CTA's k order (whole 64-k rows of its 32 weight rows),
         // so it pays for the barrier traffic of a k-block only every other k-block.
@@ -855,12 +872,26 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap
                     const uint4 pk = lds128(raw_row + xoff[chunk]);
                     w[4 * i] = pk.x; w[4 * i + 1] = pk.y; w[4 * i + 2] = pk.z; w[4 * i + 3] = pk.w;
                 }
-                const int gi = one_group ? 0
-                               : (kbg_shift >= 0 ? (kb_begin + kb) >> kbg_shift : (kb_begin + kb) / kbg) - g_first;
-                const uint32_t sz = RAW ? 0u : lds32(tbl0 + (uint32_t)(gi * BN + row) * 4u);
-                __half2 s2 = __half2half2(__ushort_as_half((unsigned short)(sz & 0xFFFFu)));
+                // scale | zero << 16 of the k-block's first and second half.  Past K both are zero: the activations are
+                // zero there (filled by TMA), and 0 x 0 adds nothing whatever the last group's scale is.
+                uint32_t sz = 0u, sz_b = 0u;
+                if (!RAW) {
+                    const int hb = 2 * (kb_begin + kb);
+                    const int gi = one_group ? 0 : (hpg_shift >= 0 ? hb >> hpg_shift : hb / hpg) - g_first;
+                    sz = sz_b = lds32(tbl0 + (uint32_t)(gi * BN + row) * 4u);
+                    if (p.half_blocks) {
+                        if ((hb + 1) * (BK / 2) >= p.K) sz_b = 0u;
+                        else if (!one_group) {
+                            const int gb = (hpg_shift >= 0 ? (hb + 1) >> hpg_shift : (hb + 1) / hpg) - g_first;
+                            sz_b = lds32(tbl0 + (uint32_t)(gb * BN + row) * 4u);
+                        }
+                    }
+                }
                 // -z with the sign flipped in place (exact)
-                __half2 nz2 = __half2half2(__ushort_as_half((unsigned short)((sz >> 16) ^ 0x8000u)));
+                const __half2 s2[2] = {__half2half2(__ushort_as_half((unsigned short)(sz & 0xFFFFu))),
+                                       __half2half2(__ushort_as_half((unsigned short)(sz_b & 0xFFFFu)))};
+                const __half2 nz2[2] = {__half2half2(__ushort_as_half((unsigned short)((sz >> 16) ^ 0x8000u))),
+                                        __half2half2(__ushort_as_half((unsigned short)((sz_b >> 16) ^ 0x8000u)))};
                 if (i >= S) {   // the MMAs that read this ring slot S k-blocks ago are done
                     if (!bar_wait(done0 + 8 * wd, wph)) { failed = true; break; }
                     wd += wstep;
@@ -869,13 +900,21 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap
                 const uint32_t a_row = tiles + s * A_STAGE + row * 128;
                 if constexpr (SPLIT) {
                     // scale and -zero as fp32, from whichever 16-bit type the table holds
-                    float s32, nz32;
+                    float s32[2], nz32[2];
                     if (p.scale_dtype == MNQ_BF16) {
-                        s32 = __uint_as_float(sz << 16);
-                        nz32 = -__uint_as_float(sz & 0xFFFF0000u);
+                        s32[0] = __uint_as_float(sz << 16);
+                        nz32[0] = -__uint_as_float(sz & 0xFFFF0000u);
+                        s32[1] = __uint_as_float(sz_b << 16);
+                        nz32[1] = -__uint_as_float(sz_b & 0xFFFF0000u);
                     } else {
-                        s32 = __half2float(__ushort_as_half((unsigned short)(sz & 0xFFFFu)));
-                        nz32 = -__half2float(__ushort_as_half((unsigned short)(sz >> 16)));
+                        s32[0] = __half2float(__ushort_as_half((unsigned short)(sz & 0xFFFFu)));
+                        nz32[0] = -__half2float(__ushort_as_half((unsigned short)(sz >> 16)));
+                        s32[1] = __half2float(__ushort_as_half((unsigned short)(sz_b & 0xFFFFu)));
+                        nz32[1] = -__half2float(__ushort_as_half((unsigned short)(sz_b >> 16)));
+                    }
+                    if (HSPLIT) {   // (exact)
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) { s32[h] *= row_down; nz32[h] *= row_down; }
                     }
                     if constexpr (TA) {
                         // this thread's row of both tiles: 32 + 32 columns of its tensor-memory lane
@@ -883,8 +922,8 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap
 #pragma unroll
                         for (int c = 0; c < 8; c += 2) {
                             uint4 hi0, lo0, hi1, lo1;
-                            split_chunk<QUANT>(&w[c * SplitChunk<QUANT>::WORDS], s32, nz32, hi0, lo0);
-                            split_chunk<QUANT>(&w[(c + 1) * SplitChunk<QUANT>::WORDS], s32, nz32, hi1, lo1);
+                            split_chunk<QUANT, HSPLIT>(&w[c * SplitChunk<QUANT>::WORDS], s32[c >> 2], nz32[c >> 2], hi0, lo0);
+                            split_chunk<QUANT, HSPLIT>(&w[(c + 1) * SplitChunk<QUANT>::WORDS], s32[c >> 2], nz32[c >> 2], hi1, lo1);
                             tmem_st8(a_t + 4 * c, hi0, hi1);
                             tmem_st8(a_t + 32 + 4 * c, lo0, lo1);
                         }
@@ -894,7 +933,7 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap
 #pragma unroll
                         for (int c = 0; c < 8; ++c) {
                             uint4 hi, lo;
-                            split_chunk<QUANT>(&w[c * SplitChunk<QUANT>::WORDS], s32, nz32, hi, lo);
+                            split_chunk<QUANT, HSPLIT>(&w[c * SplitChunk<QUANT>::WORDS], s32[c >> 2], nz32[c >> 2], hi, lo);
                             sts128(a_row + xoff[c], hi);
                             sts128(a_row + A_BYTES + xoff[c], lo);
                         }
@@ -905,8 +944,8 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap
                     const uint32_t a_t = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(p.tmem_a_col + s * A_COLS);
 #pragma unroll
                     for (int c = 0; c < 8; c += 2) {
-                        const uint4 o0 = Chunk::run(&w[c * Chunk::WORDS], s2, nz2);
-                        const uint4 o1 = Chunk::run(&w[(c + 1) * Chunk::WORDS], s2, nz2);
+                        const uint4 o0 = Chunk::run(&w[c * Chunk::WORDS], s2[c >> 2], nz2[c >> 2]);
+                        const uint4 o1 = Chunk::run(&w[(c + 1) * Chunk::WORDS], s2[c >> 2], nz2[c >> 2]);
                         tmem_st8(a_t + 4 * c, o0, o1);
                     }
                     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -915,7 +954,7 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap
 #pragma unroll
                     for (int c = 0; c < 8; ++c) {
                         using Chunk = TileChunk<QUANT, TileT>;
-                        const uint4 o = Chunk::run(&w[c * Chunk::WORDS], s2, nz2);
+                        const uint4 o = Chunk::run(&w[c * Chunk::WORDS], s2[c >> 2], nz2[c >> 2]);
                         sts128(a_row + xoff[c], o);
                     }
                 }
@@ -954,10 +993,8 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap
             float scale = 1.f, zterm = 0.f;
             if (p.epilogue_scale) scale = widen16(p.scales, sc_row, p.scale_dtype);
             const float* tscale = nullptr;
-            if (HALF_T) {   // the tile was built from scales and zeros divided by the row's 2^E
-                scale = row_up[row];
-                tscale = p.tok_scale;
-            }
+            if (HALF_T || HSPLIT) scale = row_up[row];   // the tile was built from scales and zeros divided by the row's 2^E
+            if (HALF_T) tscale = p.tok_scale;
             if (RAW) {
                 const float s_n = scale;
                 scale = s_n * 16777216.f;
@@ -1144,7 +1181,8 @@ struct GemmPlan {
     size_t smem;
 };
 
-constexpr int kMaxTableGroups = 64;   // 32 KB of scale table at most
+constexpr int kMaxTableGroups = 64;   // 32 KB of scale table at most ...
+constexpr int kMaxTableGroupsOdd = 136;   // ... and 68 KB for the small groups that only come with two tiles per k-block
 
 // K splits: the count that minimises waves x (k-blocks per split + fixed per-CTA cost) plus
 // the cost of writing and re-reading one fp32 result plane per split and of the second
@@ -1259,23 +1297,31 @@ bool tile_plan(int64_t M, int64_t N, int variant, GemmPlan* out)
     return true;
 }
 
+// Two 16-bit tiles per k-block (hi + lo), unless raw-integer tiles apply.
+inline bool two_tiles(const MatmulArgs& a, bool raw)
+{
+    if (raw) return false;
+    return a.act_dtype == MNQ_BF16 ? a.group_size < a.K || a.zeros != nullptr : odd_halves(a.K, a.group_size);
+}
+
 bool plan_gemm(const MatmulArgs& a, const mnq_tuning* tuning, GemmPlan* out)
 {
-    if (a.M < 1 || a.N < 1 || a.K < BK || a.K % BK) return false;
+    if (a.M < 1 || a.N < 1 || a.K < BK || a.K % (BK / 2)) return false;
     if (a.K > (1 << 28) || a.N > (1 << 30) || a.M > (1 << 24)) return false;
     if (reinterpret_cast<uintptr_t>(a.wq) % 16 || reinterpret_cast<uintptr_t>(a.x) % 16 || a.lda % 8) return false;
-    if (a.group_size < a.K && a.group_size % BK) return false;
+    if (a.group_size < a.K && a.group_size % (BK / 2)) return false;
     if (a.act_dtype == MNQ_FP16 && a.scale_dtype != MNQ_FP16 && !raw_applicable(a.M, a.K, a.group_size, a.quant))
         return false;   // the fp16 tile math is fp16 x fp16
     // int8 with one scale per row, few tokens: raw-integer tiles (variant 5 forbids them); their workspace
     // need is checked once the K split is known
     bool raw = raw_applicable(a.M, a.K, a.group_size, a.quant) && !(tuning && tuning->gemv_variant == 5) &&
                (a.act_dtype == MNQ_BF16 || a.scale_dtype == MNQ_FP16 || a.scale_dtype == MNQ_BF16);
-    // bf16 activations otherwise: integer tile when one scale per row and no zeros, else two bf16 tiles per k-block
-    bool split_tiles = !raw && a.act_dtype == MNQ_BF16 && (a.group_size < a.K || a.zeros != nullptr);
+    // bf16 activations otherwise: integer tile when one scale per row and no zeros, else two bf16 tiles per k-block;
+    // fp16 activations: two fp16 tiles for groups or rows of an odd number of 32s
+    bool split_tiles = two_tiles(a, raw);
     // ... or, if the caller opted in (MNQ_OPT_BF16_FP16_TILES) and the workspace can hold an fp16 copy of the
     // activations, one fp16 tile (HalfTile; variant 8 forbids it); checked again once the K split is known
-    bool half_tiles = split_tiles && option_value(MNQ_OPT_BF16_FP16_TILES) != 0 && !(tuning && tuning->gemv_variant == 8) &&
+    bool half_tiles = split_tiles && a.act_dtype == MNQ_BF16 && option_value(MNQ_OPT_BF16_FP16_TILES) != 0 && !(tuning && tuning->gemv_variant == 8) &&
                       a.workspace &&
                       a.workspace_bytes >= raw_region_offset(1, a.M, a.N) + raw_region_bytes(a.M, a.K, true);
     if (half_tiles) split_tiles = false;
@@ -1283,7 +1329,7 @@ bool plan_gemm(const MatmulArgs& a, const mnq_tuning* tuning, GemmPlan* out)
     GemmPlan pl{};
     if (!tile_plan(a.M, a.N, tuning ? tuning->gemv_variant : 0, &pl)) return false;
 
-    const int num_kb = static_cast<int>(a.K / BK);
+    const int num_kb = static_cast<int>((a.K + BK - 1) / BK);
     const int64_t tiles = static_cast<int64_t>(pl.tiles_n) * pl.tiles_m;
     // two CTAs per SM where a CTA needs at most half of everything (variant 3 forbids it)
     const bool occ2_ok = !pl.pair && pl.tmem_cols <= 256 && !split_tiles && !(tuning && tuning->gemv_variant == 3);
@@ -1297,7 +1343,8 @@ bool plan_gemm(const MatmulArgs& a, const mnq_tuning* tuning, GemmPlan* out)
         --best;   // not enough workspace: fewer splits (one split needs none)
     // the scale table holds at most kMaxTableGroups groups per row: split K further if needed
     const int64_t total_groups = a.group_size >= a.K ? 1 : (a.K + a.group_size - 1) / a.group_size;
-    const int min_splits = static_cast<int>((total_groups + kMaxTableGroups - 1) / kMaxTableGroups);
+    const int max_table = odd_halves(a.K, a.group_size) ? kMaxTableGroupsOdd : kMaxTableGroups;
+    const int min_splits = static_cast<int>((total_groups + max_table - 1) / max_table);
     if (best < min_splits) best = min_splits;
     if (best > kMaxSplits || best > num_kb) return false;
     if (best > 1 && split_workspace_bytes(best, a.M, a.N) > (a.workspace ? a.workspace_bytes : 0)) return false;
@@ -1308,7 +1355,7 @@ bool plan_gemm(const MatmulArgs& a, const mnq_tuning* tuning, GemmPlan* out)
         // not enough workspace for the prepared activations: the dequantising tile path
         raw = false;
         if (a.act_dtype == MNQ_FP16 && a.scale_dtype != MNQ_FP16) return false;
-        split_tiles = a.act_dtype == MNQ_BF16 && (a.group_size < a.K || a.zeros != nullptr);
+        split_tiles = two_tiles(a, false);
         a_stage = split_tiles ? 2 * A_BYTES : A_BYTES;
     }
     if (half_tiles && raw_region_offset(pl.splits, a.M, a.N) + raw_region_bytes(a.M, a.K, true) > a.workspace_bytes) {
@@ -1429,7 +1476,7 @@ int launch_gemm_one(const GemmParams& p, const CUtensorMap& xmap, const CUtensor
                     bool pair, bool occ2, bool ta, cudaStream_t stream)
 {
     auto* kern = pair ? &gemm_tcgen05_kernel<QUANT, T, TT, true, false> : &gemm_tcgen05_kernel<QUANT, T, TT, false, false>;
-    if constexpr (!std::is_same<TT, BSplit>::value) {
+    if constexpr (!std::is_same<TT, BSplit>::value && !std::is_same<TT, HSplit>::value) {
         if (occ2 && !pair) kern = &gemm_tcgen05_kernel<QUANT, T, TT, false, true>;
         if (ta && !pair) kern = occ2 ? &gemm_tcgen05_kernel<QUANT, T, TT, false, true, true> : &gemm_tcgen05_kernel<QUANT, T, TT, false, false, true>;
     } else {
@@ -1535,7 +1582,7 @@ bool gemm_supported(const MatmulArgs& a)
 size_t gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, int32_t group_size, int32_t quant)
 {
     const size_t base = gemm_split_workspace_bytes(M, N, K, group_size);
-    if (M < 1 || N < 1 || K < BK || K % BK) return base;
+    if (M < 1 || N < 1 || K < BK || K % (BK / 2)) return base;
     // room for the prepared activations (raw-integer tiles; fp16 tiles for bf16 activations if the caller opted
     // in): per-token factor and sum and, sized for bf16 activations, their fp16 copy
     // the tail cut's planes (whichever occupancy the plan ends up with), after the prepared activations if any
@@ -1545,7 +1592,7 @@ size_t gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, int32_t group_size,
         if (base <= kCounterBytes && tile_plan(M, N, 0, &pl) && !pl.pair && pl.tiles_m == 1)
             for (int per_sm = 1; per_sm <= 2; ++per_sm) {
                 int from = -1;
-                const int ts = choose_tail(pl.tiles_n, static_cast<int>(K / BK), 148 * per_sm, M, &from);
+                const int ts = choose_tail(pl.tiles_n, static_cast<int>((K + BK - 1) / BK), 148 * per_sm, M, &from);
                 if (ts > 1) tail = std::max(tail, tail_bytes(ts, M, N, from) + 256);
             }
     }
@@ -1559,15 +1606,19 @@ size_t gemm_split_workspace_bytes(int64_t M, int64_t N, int64_t K, int32_t group
 {
     // What plan_gemm asks for on a 148-SM part (B200).  On a device where it would split
     // further, the plan falls back to the number of splits the given workspace can hold.
-    if (M < 1 || N < 1 || K < BK || K % BK) return 0;
+    if (M < 1 || N < 1 || K < BK || K % (BK / 2)) return 0;
     GemmPlan pl{};
     if (!tile_plan(M, N, 0, &pl)) return 0;
     const int64_t tiles = static_cast<int64_t>(pl.tiles_n) * pl.tiles_m;
     int occ2 = 0;   // as plan_gemm
-    int splits = choose_occupancy_and_splits(!pl.pair && pl.tmem_cols <= 256, tiles, static_cast<int>(K / BK), 148,
+    int splits = choose_occupancy_and_splits(!pl.pair && pl.tmem_cols <= 256, tiles, static_cast<int>((K + BK - 1) / BK), 148,
                                              4.0 * M * N, &occ2);
+    const bool odd = odd_halves(K, group_size);
+    if (odd)   // (two tiles per k-block never run two CTAs per SM)
+        splits = std::max(splits, choose_occupancy_and_splits(false, tiles, static_cast<int>((K + BK - 1) / BK), 148, 4.0 * M * N, &occ2));
     const int64_t total_groups = group_size >= K ? 1 : (K + group_size - 1) / group_size;
-    const int min_splits = static_cast<int>((total_groups + kMaxTableGroups - 1) / kMaxTableGroups);
+    const int max_table = odd ? kMaxTableGroupsOdd : kMaxTableGroups;
+    const int min_splits = static_cast<int>((total_groups + max_table - 1) / max_table);
     if (splits < min_splits) splits = min_splits;
     if (splits <= 1 || splits > kMaxSplits) return 0;
     return split_workspace_bytes(splits, M, N);
@@ -1578,18 +1629,20 @@ int launch_gemm(const MatmulArgs& a, const mnq_tuning* tuning)
     GemmPlan pl;
     if (!plan_gemm(a, tuning, &pl))
         return fail(MNQ_INVALID_ARGUMENT, "dequant_matmul: the tensor-core kernel cannot take this problem "
-                                          "(needs K % 64 == 0, 16-byte aligned operands, group_size % 64 == 0 or >= K, "
+                                          "(needs K % 32 == 0, K >= 64, 16-byte aligned operands, group_size % 32 == 0 or >= K, "
                                           "fp16 scales with fp16 activations)");
     GemmParams p{};
     p.wq = static_cast<const uint8_t*>(a.wq); p.scales = a.scales; p.zeros = a.zeros; p.out = a.out;
     p.M = static_cast<int>(a.M); p.N = static_cast<int>(a.N); p.K = static_cast<int>(a.K);
     p.ldc = a.ldc;
+    p.kb_total = static_cast<int>((a.K + BK - 1) / BK);
+    p.half_blocks = (a.K % BK != 0 || (a.group_size < a.K && a.group_size % BK != 0)) ? 1 : 0;
     p.row_bytes = static_cast<int>(a.quant == MNQ_INT4 ? a.K / 2 : a.K);
     p.group_size = a.group_size; p.G = a.G; p.scale_dtype = a.scale_dtype;
     p.tok = pl.tok; p.tokh = pl.tokh; p.nh = pl.nh; p.stages = pl.stages; p.b_stages = pl.b_stages;
     p.raw_stages = pl.raw_stages; p.raw_segs = pl.raw_segs; p.commit_every = pl.commit_every; p.table_groups = pl.table_groups; p.tmem_cols = pl.tmem_cols;
     p.tmem_a_col = pl.tmem_a_col;
-    const bool split_tiles = !pl.raw && !pl.half && a.act_dtype == MNQ_BF16 && (a.group_size < a.K || a.zeros != nullptr);
+    const bool split_tiles = !pl.half && two_tiles(a, pl.raw != 0);
     p.epilogue_scale = (a.act_dtype == MNQ_BF16 && !split_tiles && !pl.half) ? 1 : 0;
     p.splits = pl.splits; p.kb_per_split = pl.kb_per_split;
     p.vec_store = ((reinterpret_cast<uintptr_t>(a.out) % 16 == 0 && a.ldc % 8 == 0) ? 1 : 0) | ((a.N % 4 == 0) ? 2 : 0) |
@@ -1663,10 +1716,12 @@ int launch_gemm(const MatmulArgs& a, const mnq_tuning* tuning)
         return launch_gemm_one<MNQ_INT8, __nv_bfloat16, HalfTile>(p, xmap, wmap, grid, pl.smem, pair, pl.occ2 != 0, pl.ta != 0, a.stream);
     }
     if (a.quant == MNQ_INT4) {
+        if (a.act_dtype == MNQ_FP16 && split_tiles) return launch_gemm_one<MNQ_INT4, __half, HSplit>(p, xmap, wmap, grid, pl.smem, pair, pl.occ2 != 0, pl.ta != 0, a.stream);
         if (a.act_dtype == MNQ_FP16) return launch_gemm_one<MNQ_INT4, __half, __half>(p, xmap, wmap, grid, pl.smem, pair, pl.occ2 != 0, pl.ta != 0, a.stream);
         if (split_tiles) return launch_gemm_one<MNQ_INT4, __nv_bfloat16, BSplit>(p, xmap, wmap, grid, pl.smem, pair, pl.occ2 != 0, pl.ta != 0, a.stream);
         return launch_gemm_one<MNQ_INT4, __nv_bfloat16, __nv_bfloat16>(p, xmap, wmap, grid, pl.smem, pair, pl.occ2 != 0, pl.ta != 0, a.stream);
     }
+    if (a.act_dtype == MNQ_FP16 && split_tiles) return launch_gemm_one<MNQ_INT8, __half, HSplit>(p, xmap, wmap, grid, pl.smem, pair, pl.occ2 != 0, pl.ta != 0, a.stream);
     if (a.act_dtype == MNQ_FP16) return launch_gemm_one<MNQ_INT8, __half, __half>(p, xmap, wmap, grid, pl.smem, pair, pl.occ2 != 0, pl.ta != 0, a.stream);
     if (split_tiles) return launch_gemm_one<MNQ_INT8, __nv_bfloat16, BSplit>(p, xmap, wmap, grid, pl.smem, pair, pl.occ2 != 0, pl.ta != 0, a.stream);
     return launch_gemm_one<MNQ_INT8, __nv_bfloat16, __nv_bfloat16>(p, xmap, wmap, grid, pl.smem, pair, pl.occ2 != 0, pl.ta != 0, a.stream);

@@ -282,6 +282,9 @@ struct MatmulArgs {
 inline int64_t packed_weight_bytes(const MatmulArgs& a) { return a.N * (a.quant == MNQ_INT4 ? a.K / 2 : a.K); }
 inline bool few_rows_small_layer(const MatmulArgs& a) { return a.N < 8192 && packed_weight_bytes(a) < (int64_t(24) << 20); }
 
+// Groups, or rows, of an odd number of 32s.
+inline bool odd_halves(int64_t K, int64_t group_size) { return K % 64 != 0 || (group_size < K && group_size % 64 != 0); }
+
 // Process-wide options (mnq_set_option); defined in api.cu.
 int64_t option_value(int option);
 

@@ -61,7 +61,11 @@ int mnq_dequant_matmul_static(const void* activations, const void* weights_packe
                               int32_t scale_dtype, void* stream)
 {
     // Problems whose split-K scratch would not fit are refused, not silently run slower.
-    const size_t need = mnq_workspace_bytes(M, N, K, group_size, quant_type);
+    size_t need = mnq_workspace_bytes(M, N, K, group_size, quant_type);
+    // (The tensor-core kernel takes rows of an odd number of 32s with whatever scratch there is, or leaves them to the any-shape
+    // kernel, which needs none.)
+    if (need > kStaticScratchBytes && K % 64 != 0 && (M > 64 || gemv_workspace_bytes(M, N, K, group_size, quant_type) <= kStaticScratchBytes))
+        need = kStaticScratchBytes;
     if (need > kStaticScratchBytes)
         return fail(MNQ_INVALID_ARGUMENT,
                     "dequant_matmul_static: this problem wants %zu bytes of scratch, the built-in area holds %zu "

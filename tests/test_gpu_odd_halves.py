@@ -1,0 +1,72 @@
+"""Groups, or rows, of an odd number of 32s on the tensor-core kernel, against the CPU oracle and against the any-shape
+kernel, which keeps every weight in fp32."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import check as H
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def mn():
+    import metal_native
+    assert torch.cuda.is_available()
+    return metal_native
+
+
+CASES = [
+    # quant, M, N, K, g, zeros, act dtype, scale dtype, K splits (0: the plan's)
+    ("int4", 16, 128, 64, 32, True, torch.float16, torch.float16, 0),       # one k-block, two groups
+    ("int4", 33, 130, 96, 32, True, torch.float16, torch.float16, 0),       # half a k-block at the end, ragged rows
+    ("int4", 64, 256, 1056, 32, False, torch.float16, torch.float16, 0),    # odd number of groups a row
+    ("int4", 100, 200, 960, 96, True, torch.bfloat16, torch.bfloat16, 0),   # groups of three halves
+    ("int4", 128, 300, 4096, 32, True, torch.float16, torch.float16, 0),    # weight tiles in tensor memory, 64-column slots
+    ("int4", 129, 300, 4096, 32, True, torch.bfloat16, torch.float16, 0),   # ... and in shared memory
+    ("int4", 197, 515, 4160, 32, True, torch.float16, torch.float16, 0),
+    ("int4", 300, 384, 1024, 32, True, torch.float16, torch.float16, 3),    # CTA pairs, K splits
+    ("int4", 70, 384, 2080, 2080, True, torch.bfloat16, torch.bfloat16, 2), # one group per row, with zeros
+    ("int4", 70, 384, 2080, 2080, False, torch.bfloat16, torch.bfloat16, 2),  # integer tile
+    ("int8", 48, 140, 1120, 160, True, torch.float16, torch.float16, 0),    # groups of five halves
+    ("int8", 200, 256, 672, 672, True, torch.bfloat16, torch.float16, 0),   # raw-integer tiles
+    ("int8", 520, 384, 672, 672, False, torch.float16, torch.float16, 0),   # more tokens than those take
+    ("int4", 40, 256, 9632, 32, True, torch.float16, torch.float16, 0),     # more groups than one table holds
+]
+
+
+@pytest.mark.parametrize("quant,M,N,K,g,zeros,adt,sdt,split", CASES)
+def test_odd_halves(mn, quant, M, N, K, g, zeros, adt, sdt, split):
+    import mnq_workloads as workloads
+    C = mn._C
+    L = workloads.make_layer("t", M, K, N, quant_type=quant, group_size=g, act_dtype=adt, scale_dtype=sdt,
+                             asymmetric=zeros, seed=M + N + K)
+    if g == 32 and sdt == torch.float16 and N == 300:   # rows whose scales lie far apart
+        L.scales[::2] *= 2.0 ** -6
+    ref = H.oracle_matmul(L)
+    d = L.to("cuda")
+    t = C.Tuning()
+    t.path, t.split_k = C.PATH_GEMM, split
+    buf = torch.full((M + 2, N + 8), 777.0, dtype=adt, device="cuda")
+    out = buf[1:M + 1, 3:N + 3]
+    C.dequant_matmul(*d.args(), out=out, tuning=t)
+    again = C.dequant_matmul(*d.args(), tuning=t)
+    t.path, t.split_k = C.PATH_GENERIC, 0
+    fp32_weights = C.dequant_matmul(*d.args(), tuning=t)
+    C.synchronize()
+    assert C.device_status() == 0
+    H.assert_close_to_oracle(out, ref, f"{quant} {M}x{N}x{K} g{g}")
+    assert torch.equal(out, again)
+    chk = buf.clone()
+    chk[1:M + 1, 3:N + 3] = 777.0
+    assert bool((chk == 777.0).all()), "kernel wrote outside its [M, N] output block"
+    # no further from the oracle than fp32 weights: both errors are the rounding of the output, up to ties
+    err = [float(np.linalg.norm(y.float().cpu().numpy() - ref) / np.linalg.norm(ref)) for y in (out, fp32_weights)]
+    assert err[0] <= err[1] * 1.01, err
+
+
+def test_dispatch(mn):
+    sp = mn._C.select_path
+    assert sp(197, 5003, 4160, 32, "int4") == "gemm"
+    assert sp(64, 4096, 4128, 4128, "int8", torch.bfloat16, zeros=False) == "gemm"
+    assert sp(64, 4096, 4112, 4112, "int8", torch.bfloat16, zeros=False) == "generic"   # no multiple of 32
