@@ -257,7 +257,7 @@ int choose_path(const MatmulArgs& a)
         return MNQ_PATH_GEMV;
     // (a problem of a few million products with groups or rows of an odd number of 32s is over in the any-shape kernel
     // before the tensor-core kernel has set up: 1.3 million (K, N, M = 160, 256, 33) 4.5 us, 7.3 million 11.0 against 6.8,
-    // 4.2 billion 3570 against 52)
+    // 4.2 billion 3570 against 45)
     if (a.M > gemv_max_m && gemm_supported(a) && !(odd_halves(a.K, a.group_size) && a.M * a.N * a.K < kAnyShapeProducts))
         return MNQ_PATH_GEMM;
     if (a.M <= 32 && gemv_supported(a)) return MNQ_PATH_GEMV;   // e.g. K not a multiple of 64

@@ -565,6 +565,11 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap
     constexpr int KB_BYTES = WPK * 32;                  // packed bytes per row per k-block
     constexpr int KPR = 128 / KB_BYTES;                 // k-blocks covered by one raw stage (128 packed bytes per row)
     constexpr int RAW_BYTES = BN * 128;
+    // The k-blocks of a packed stage as a loop for int4 (four of them; the expanded body is 150 to 450 instructions, and
+    // four copies of it ran from beyond the instruction caches: half of all stalls were for instructions), unrolled for
+    // int8 (two short ones).  Measured, K = 4096, N = 14336, int4: two bf16 tiles at 128 tokens 67 -> 41 us, one fp16 tile
+    // at 256 tokens 40 -> 34, groups of 32 at 64 tokens 112 -> 79; int8 as a loop: 24 -> 25.
+    constexpr int KB_UNROLL = QUANT == MNQ_INT4 ? 1 : KPR;
     constexpr bool IS_BF16 = std::is_same<T, __nv_bfloat16>::value;
     constexpr bool HSPLIT = std::is_same<TT, HSplit>::value;
     constexpr bool SPLIT = std::is_same<TT, BSplit>::value || HSPLIT;   // two tiles per k-block
@@ -859,7 +864,7 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap
             const int jj = st + j < num_raw ? st + j : st + j - num_raw;
             for (int u = 0; u < NSEG && !failed; ++u) {
             const uint32_t raw_row = raw0 + (r * NSEG + u) * RAW_BYTES + row * 128;
-#pragma unroll
+#pragma unroll KB_UNROLL
             for (int q = 0; q < KPR; ++q) {
                 const int kb = (jj * NSEG + u) * KPR + q;
                 if (kb >= num_kb || failed) break;
@@ -869,7 +874,7 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap
 #pragma unroll
                 for (int i = 0; i < 2 * WPK; ++i) {
                     const int chunk = q * (8 / KPR) + i;   // 16-byte chunk of the 128-byte raw row
-                    const uint4 pk = lds128(raw_row + xoff[chunk]);
+                    const uint4 pk = lds128(raw_row + (KB_UNROLL == 1 ? ((uint32_t)chunk << 4) ^ xoff[0] : xoff[chunk]));
                     w[4 * i] = pk.x; w[4 * i + 1] = pk.y; w[4 * i + 2] = pk.z; w[4 * i + 3] = pk.w;
                 }
                 // scale | zero << 16 of the k-block's first and second half.  Past K both are zero: the activations are
@@ -879,7 +884,7 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap
                     const int hb = 2 * (kb_begin + kb);
                     const int gi = one_group ? 0 : (hpg_shift >= 0 ? hb >> hpg_shift : hb / hpg) - g_first;
                     sz = sz_b = lds32(tbl0 + (uint32_t)(gi * BN + row) * 4u);
-                    if (p.half_blocks) {
+                    if (SPLIT && p.half_blocks) {   // (one tile of scaled weights never meets them, and was 5 % slower with the test)
                         if ((hb + 1) * (BK / 2) >= p.K) sz_b = 0u;
                         else if (!one_group) {
                             const int gb = (hpg_shift >= 0 ? (hb + 1) >> hpg_shift : (hb + 1) / hpg) - g_first;
@@ -1321,7 +1326,7 @@ bool plan_gemm(const MatmulArgs& a, const mnq_tuning* tuning, GemmPlan* out)
     bool split_tiles = two_tiles(a, raw);
     // ... or, if the caller opted in (MNQ_OPT_BF16_FP16_TILES) and the workspace can hold an fp16 copy of the
     // activations, one fp16 tile (HalfTile; variant 8 forbids it); checked again once the K split is known
-    bool half_tiles = split_tiles && a.act_dtype == MNQ_BF16 && option_value(MNQ_OPT_BF16_FP16_TILES) != 0 && !(tuning && tuning->gemv_variant == 8) &&
+    bool half_tiles = split_tiles && a.act_dtype == MNQ_BF16 && !odd_halves(a.K, a.group_size) && option_value(MNQ_OPT_BF16_FP16_TILES) != 0 && !(tuning && tuning->gemv_variant == 8) &&
                       a.workspace &&
                       a.workspace_bytes >= raw_region_offset(1, a.M, a.N) + raw_region_bytes(a.M, a.K, true);
     if (half_tiles) split_tiles = false;
