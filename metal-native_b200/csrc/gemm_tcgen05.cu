@@ -463,13 +463,15 @@ template <> struct StageIO<__nv_bfloat16> {
 // T: the activation type (what bias and residual hold).  FINAL: the values stored are the
 // operator's result, so the epilogue is applied while they are staged; otherwise (a K split's
 // fp32 plane) they are stored as they are.
-// tok_scale / tok_sum / zterm: raw-integer tiles only (tok_scale == nullptr otherwise): the value of token m is
-// acc * scale * tok_scale[m] - zterm * tok_sum[m].
-template <typename E, typename T, bool FINAL>
+// TOK: prepared activations (raw-integer tiles, HalfTile): the value of the tile's token c is acc * scale * f[c], with
+// f the `tok` floats at shared address tok_at, and for raw-integer tiles (SUMS) - zterm * x[c], x the `tok` floats after
+// them.  (Read from global memory, two loads and a clamp for every element, they made the epilogue of 512 tokens x 128
+// rows last 35 us: [512, 4096] x [14336, 4096] int4 bf16 as one fp16 tile 86 us, from shared memory 55.)
+constexpr int kSlabBytes = 2 * 64 * BN * 4;   // the two staging buffers at their largest; the per-token factors lie behind them
+template <typename E, typename T, bool FINAL, bool TOK, bool SUMS>
 __device__ __forceinline__ void epilogue_tile(uint32_t tmem_base, int quad, int half, int row, int e, int tok,
                                               uint32_t stage0, float scale, E* dst, size_t ld, int n0, int N, int m0,
-                                              int M, bool vec, const Epilogue& epi, const float* tok_scale = nullptr,
-                                              const float* tok_sum = nullptr, float zterm = 0.f)
+                                              int M, bool vec, const Epilogue& epi, uint32_t tok_at, float zterm)
 {
     constexpr int RB = BN * (int)sizeof(E);    // bytes per staged token row
     constexpr int PPR = RB / 16;               // 16-byte pieces per row
@@ -484,14 +486,31 @@ __device__ __forceinline__ void epilogue_tile(uint32_t tmem_base, int quad, int 
             tmem_ld32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, v);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             const uint32_t at = stage + (uint32_t)(half * 32 * RB) + (uint32_t)row * (uint32_t)sizeof(E);
-            if (tok_scale) {
+            if (TOK) {
                 const bool n_ok = n0 + row < N;
 #pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    const int m = min(m0 + c0 + i, M - 1);
-                    float val = fmaf(-zterm, __ldg(tok_sum + m), __uint_as_float(v[i]) * scale * __ldg(tok_scale + m));
-                    if (FINAL && n_ok && m0 + c0 + i < M) val = epilogue_value<T>(epi, val, m0 + c0 + i, n0 + row);
-                    StageIO<E>::put(at + i * RB, StageIO<E>::from(val));
+                for (int i = 0; i < 32; i += 4) {
+                    const uint4 f = lds128(tok_at + (uint32_t)((c0 + i) * 4));
+                    uint4 x = make_uint4(0u, 0u, 0u, 0u);
+                    if (SUMS) x = lds128(tok_at + (uint32_t)((tok + c0 + i) * 4));
+                    const uint32_t fw[4] = {f.x, f.y, f.z, f.w}, xw[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        float val = __uint_as_float(v[i + k]) * scale * __uint_as_float(fw[k]);
+                        if (SUMS) val = fmaf(-zterm, __uint_as_float(xw[k]), val);
+                        v[i + k] = __float_as_uint(val);
+                    }
+                }
+                if (FINAL && epi.kind != MNQ_EPI_NONE) {
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) {
+                        float val = __uint_as_float(v[i]);
+                        if (n_ok && m0 + c0 + i < M) val = epilogue_value<T>(epi, val, m0 + c0 + i, n0 + row);
+                        StageIO<E>::put(at + i * RB, StageIO<E>::from(val));
+                    }
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) StageIO<E>::put(at + i * RB, StageIO<E>::from(__uint_as_float(v[i])));
                 }
             } else if (FINAL && epi.kind != MNQ_EPI_NONE) {
                 const bool n_ok = n0 + row < N;
@@ -980,6 +999,19 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap
             if (++r == R) { r = 0; rph ^= 1u; }
         }
 
+        // the tile's per-token factors and sums, on their way while the last MMAs run
+        constexpr bool TOK = RAW || HALF_T;
+        float tok_f[2] = {0.f, 0.f}, tok_x[2] = {0.f, 0.f};
+        if (TOK) {
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int c = tid - 64 + 256 * u, m = min(m0 + c, p.M - 1);
+                if (c < p.tok) {
+                    tok_f[u] = __ldg(p.tok_scale + m);
+                    if (RAW) tok_x[u] = __ldg(p.tok_sum + m);
+                }
+            }
+        }
         // epilogue: accumulator row `row` holds out[m0 .. m0+tok, n]; this warp takes the
         // 32-column chunks with chunk index % 2 == half
         if (!failed && !bar_wait(accum, 0)) failed = true;
@@ -997,34 +1029,43 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             float scale = 1.f, zterm = 0.f;
             if (p.epilogue_scale) scale = widen16(p.scales, sc_row, p.scale_dtype);
-            const float* tscale = nullptr;
+            const uint32_t tok_at = tiles + kSlabBytes;   // (the rings are idle)
+            if (TOK) {
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const int c = tid - 64 + 256 * u;
+                    if (c < p.tok) {
+                        asm volatile("st.shared.f32 [%0], %1;" ::"r"(tok_at + (uint32_t)(c * 4)), "f"(tok_f[u]) : "memory");
+                        if (RAW) asm volatile("st.shared.f32 [%0], %1;" ::"r"(tok_at + (uint32_t)((p.tok + c) * 4)), "f"(tok_x[u]) : "memory");
+                    }
+                }
+                asm volatile("bar.sync 1, 256;" ::: "memory");
+            }
             if (HALF_T || HSPLIT) scale = row_up[row];   // the tile was built from scales and zeros divided by the row's 2^E
-            if (HALF_T) tscale = p.tok_scale;
             if (RAW) {
                 const float s_n = scale;
                 scale = s_n * 16777216.f;
                 if (p.offset_term && (!cut || part == 0))
                     zterm = fmaf(128.f, s_n, p.zeros ? widen16(p.zeros, sc_row, p.scale_dtype) : 0.f);
-                tscale = p.tok_scale;
             }
             // with K split, this CTA's result goes to its [M][N] plane of the workspace instead;
             // the rings are idle now (every MMA has completed), so their memory stages the tile
             if (in_tail) {   // plane `part` of the tail's own planes, Nt = N - tail_from * 128 columns wide; indexed by the global n
                 const size_t Nt = (size_t)(p.N - p.tail_from * BN);
-                epilogue_tile<float, T, false>(tmem_base, quad, half, row, tid - 64, p.tok, tiles, scale,
+                epilogue_tile<float, T, false, TOK, RAW>(tmem_base, quad, half, row, tid - 64, p.tok, tiles, scale,
                                                p.tail_partial + (size_t)part * p.M * Nt - (size_t)p.tail_from * BN, Nt, n0, p.N, m0, p.M,
-                                               (p.vec_store & 2) != 0, p.epi, tscale, p.tok_sum, zterm);
+                                               (p.vec_store & 2) != 0, p.epi, tok_at, zterm);
             } else if (cut)
-                epilogue_tile<float, T, false>(tmem_base, quad, half, row, tid - 64, p.tok, tiles, scale,
+                epilogue_tile<float, T, false, TOK, RAW>(tmem_base, quad, half, row, tid - 64, p.tok, tiles, scale,
                                                p.partial + (size_t)part * p.M * p.N, (size_t)p.N, n0, p.N, m0, p.M,
-                                               (p.vec_store & 2) != 0, p.epi, tscale, p.tok_sum, zterm);
+                                               (p.vec_store & 2) != 0, p.epi, tok_at, zterm);
             else if (p.epi.out_f32)
-                epilogue_tile<float, T, true>(tmem_base, quad, half, row, tid - 64, p.tok, tiles, scale,
+                epilogue_tile<float, T, true, TOK, RAW>(tmem_base, quad, half, row, tid - 64, p.tok, tiles, scale,
                                               static_cast<float*>(p.out), (size_t)p.ldc, n0, p.N, m0, p.M,
-                                              (p.vec_store & 4) != 0, p.epi, tscale, p.tok_sum, zterm);
+                                              (p.vec_store & 4) != 0, p.epi, tok_at, zterm);
             else
-                epilogue_tile<T, T, true>(tmem_base, quad, half, row, tid - 64, p.tok, tiles, scale, static_cast<T*>(p.out),
-                                          (size_t)p.ldc, n0, p.N, m0, p.M, (p.vec_store & 1) != 0, p.epi, tscale, p.tok_sum, zterm);
+                epilogue_tile<T, T, true, TOK, RAW>(tmem_base, quad, half, row, tid - 64, p.tok, tiles, scale, static_cast<T*>(p.out),
+                                          (size_t)p.ldc, n0, p.N, m0, p.M, (p.vec_store & 1) != 0, p.epi, tok_at, zterm);
         }
     }
     if (failed && lane == 0) atomicOr(&g_gemm_status, 2u);
@@ -1380,7 +1421,8 @@ bool plan_gemm(const MatmulArgs& a, const mnq_tuning* tuning, GemmPlan* out)
     // of a k-block; about 60 % of what is left, they have the longer latency to hide) and weight tiles
     const size_t b_stage = static_cast<size_t>(pl.nh) * (pl.pair ? pl.tokh / 2 : pl.tokh) * 128;
     pl.raw_segs = 1;
-    const size_t epilogue_min = 1024 + 2 * 64 * BN * 4;   // the epilogue stages two 64-token slabs of fp32
+    // the epilogue stages two 64-token slabs of fp32, and per-token factors and sums of prepared activations
+    const size_t epilogue_min = 1024 + kSlabBytes + (raw || half_tiles ? static_cast<size_t>(pl.tok) * 8 : 0);
     // weight tiles in tensor memory (see the kernel): tiles of at most 128 tokens (variant 6 forbids it)
     // (two bf16 tiles per k-block take a 64-column slot)
     const bool ta_ok = !pl.pair && pl.nh == 1 && pl.tok <= 128 && !(tuning && tuning->gemv_variant == 6);
