@@ -141,6 +141,11 @@ MNQ_API const char* mnq_last_error(void);
  * concurrently need separate workspaces. */
 MNQ_API size_t mnq_workspace_bytes(int64_t M, int64_t N, int64_t K, int32_t group_size, int32_t quant_type);
 
+/* The same for a call whose types are known.  Symmetric int4 with bf16 activations and scales above the decode sizes uses
+ * more than mnq_workspace_bytes() names (an fp16 copy of the activations); with less, the call takes a slower kernel. */
+MNQ_API size_t mnq_workspace_bytes_for(int64_t M, int64_t N, int64_t K, int32_t group_size, int32_t quant_type,
+                                       int32_t act_dtype, int32_t scale_dtype, int32_t has_zeros);
+
 /* Fused dequantise + matmul.  Replaces
  *   MNTensor dequant_matmul(activations, weights_packed, scales, zeros, group_size, quant_type)
  * (include/metal_native/ops/matmul.h:77-82; host side src/ops/matmul.mm:903-1029).

@@ -236,6 +236,19 @@ int64_t gemv_max_m_for(int64_t K, int32_t group_size, int32_t quant, int32_t act
 
 // Decode kernels up to the threshold, the tensor-core kernel above it, the any-shape kernel for
 // whatever neither takes.
+// 33 to 64 tokens where one fp16 tile is exact (exact_half_tiles) and the workspace can hold the activations' copy, batched
+// decode against the tensor-core kernel: wide layers from 41 tokens (K 4096, N 14336 at 40 / 48 / 64 tokens: 28.4 / 32.1 /
+// 39.6 against 29.4 / 29.4 / 30.2 us; K 14336, N 4096 at 33 / 64: 27.9 / 38.2 against 37.5 / 38.7), small layers of few rows
+// from 33 (4096 x 4096 at 48: 31.1 against 17.2; 1024 x 1024 10.9 against 9.2; 256 x 512 a tie).  Fewer than 1024 rows keep the
+// batched kernel, which is documented and tested to take them, although it would lose there too (1000 x 4096: 26 against 13).
+bool one_half_tile_wins(const MatmulArgs& a)
+{
+    if (!exact_half_tiles(a.K, a.group_size, a.quant, a.act_dtype, a.scale_dtype, a.zeros != nullptr) ||
+        a.workspace_bytes < gemm_workspace_bytes(a.M, a.N, a.K, a.group_size, a.quant, true))
+        return false;
+    return few_rows_small_layer(a) ? a.N >= 1024 && packed_weight_bytes(a) >= (int64_t(256) << 10) : a.M > 40 && a.N >= 8192;
+}
+
 constexpr int64_t kAnyShapeProducts = 4 << 20;
 int choose_path(const MatmulArgs& a)
 {
@@ -253,7 +266,7 @@ int choose_path(const MatmulArgs& a)
     // kernel with six or eight token tiles is faster (measured: 31-50 against 70 us on the Llama-3-8B
     // shapes).  Only while the threshold is left to the library.
     if (a.M > 32 && a.M <= 64 && a.act_dtype == MNQ_BF16 && option_value(MNQ_OPT_GEMV_MAX_M) == 0 &&
-        option_value(MNQ_OPT_BF16_FP16_TILES) == 0 && a.group_size < a.K && gemv_supported(a))
+        option_value(MNQ_OPT_BF16_FP16_TILES) == 0 && a.group_size < a.K && gemv_supported(a) && !one_half_tile_wins(a))
         return MNQ_PATH_GEMV;
     // (a problem of a few million products with groups or rows of an odd number of 32s is over in the any-shape kernel
     // before the tensor-core kernel has set up: 1.3 million (K, N, M = 160, 256, 33) 4.5 us, 7.3 million 11.0 against 6.8,
@@ -310,6 +323,15 @@ int mnq_device_status(uint32_t* status, int32_t clear)
     return MNQ_SUCCESS;
 }
 
+size_t mnq_workspace_bytes_for(int64_t M, int64_t N, int64_t K, int32_t group_size, int32_t quant_type, int32_t act_dtype,
+                               int32_t scale_dtype, int32_t has_zeros)
+{
+    const size_t base = mnq_workspace_bytes(M, N, K, group_size, quant_type);
+    if (M <= 32 || !exact_half_tiles(K, group_size, quant_type, act_dtype, scale_dtype, has_zeros != 0)) return base;
+    const size_t half = gemm_workspace_bytes(M, N, K, group_size, quant_type, true);
+    return half > base ? half : base;
+}
+
 size_t mnq_workspace_bytes(int64_t M, int64_t N, int64_t K, int32_t group_size, int32_t quant_type)
 {
     if (M > 32) {   // (33 to 64 tokens of bf16 activations may take the batched-decode kernel: enough for both)
@@ -347,7 +369,7 @@ int mnq_select_path_ex(int64_t M, int64_t N, int64_t K, int64_t lda, int32_t gro
               quant_type, act_dtype, scale_dtype, nullptr, 0, nullptr);
     // the answer must not depend on how much workspace a later call brings
     a.workspace = reinterpret_cast<void*>(uintptr_t(256));
-    a.workspace_bytes = mnq_workspace_bytes(M, N, K, group_size, quant_type);
+    a.workspace_bytes = mnq_workspace_bytes_for(M, N, K, group_size, quant_type, act_dtype, scale_dtype, zeros != nullptr);
     return choose_path(a);
 }
 
@@ -543,7 +565,7 @@ __global__ void __launch_bounds__(256) stage_activations_kernel(const uint4* __r
 // output that follow the scratch must not land where a later split-K call expects zeroed counters.
 static size_t host_scratch_bytes(int64_t M, int64_t N, int64_t K, int32_t group_size, int32_t quant_type)
 {
-    const size_t need = align256(mnq_workspace_bytes(M, N, K, group_size, quant_type));
+    const size_t need = align256(mnq_workspace_bytes_for(M, N, K, group_size, quant_type, MNQ_BF16, MNQ_BF16, 0));   // whatever types come
     return need > mnq::kCounterBytes ? need : mnq::kCounterBytes;
 }
 
@@ -570,7 +592,7 @@ int mnq_dequant_matmul_host(const void* activations_host, const void* weights_pa
     // workspace: [operator scratch][activations][output]
     unsigned char* ws = static_cast<unsigned char*>(workspace);
     const size_t scratch = host_scratch_bytes(M, N, K, group_size, quant_type);
-    const size_t op_scratch = mnq_workspace_bytes(M, N, K, group_size, quant_type);
+    const size_t op_scratch = mnq_workspace_bytes_for(M, N, K, group_size, quant_type, act_dtype, scale_dtype, zeros != nullptr);
     unsigned char* x_dev = ws + scratch;
     unsigned char* out_dev = x_dev + align256(static_cast<size_t>(M) * K * 2);
     cudaStream_t st = static_cast<cudaStream_t>(stream);

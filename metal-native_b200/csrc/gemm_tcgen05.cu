@@ -1367,7 +1367,11 @@ bool plan_gemm(const MatmulArgs& a, const mnq_tuning* tuning, GemmPlan* out)
     bool split_tiles = two_tiles(a, raw);
     // ... or, if the caller opted in (MNQ_OPT_BF16_FP16_TILES) and the workspace can hold an fp16 copy of the
     // activations, one fp16 tile (HalfTile; variant 8 forbids it); checked again once the K split is known
-    bool half_tiles = split_tiles && a.act_dtype == MNQ_BF16 && !odd_halves(a.K, a.group_size) && option_value(MNQ_OPT_BF16_FP16_TILES) != 0 && !(tuning && tuning->gemv_variant == 8) &&
+    // or if it loses nothing (a forced path without the option keeps two)
+    const bool exact_half = exact_half_tiles(a.K, a.group_size, a.quant, a.act_dtype, a.scale_dtype, a.zeros != nullptr) &&
+                            !(tuning && tuning->path != MNQ_PATH_AUTO);
+    bool half_tiles = split_tiles && a.act_dtype == MNQ_BF16 && !odd_halves(a.K, a.group_size) &&
+                      (exact_half || option_value(MNQ_OPT_BF16_FP16_TILES) != 0) && !(tuning && tuning->gemv_variant == 8) &&
                       a.workspace &&
                       a.workspace_bytes >= raw_region_offset(1, a.M, a.N) + raw_region_bytes(a.M, a.K, true);
     if (half_tiles) split_tiles = false;
@@ -1626,7 +1630,7 @@ bool gemm_supported(const MatmulArgs& a)
     return plan_gemm(a, nullptr, &pl);
 }
 
-size_t gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, int32_t group_size, int32_t quant)
+size_t gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, int32_t group_size, int32_t quant, bool half_tiles)
 {
     const size_t base = gemm_split_workspace_bytes(M, N, K, group_size);
     if (M < 1 || N < 1 || K < BK || K % (BK / 2)) return base;
@@ -1643,7 +1647,7 @@ size_t gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, int32_t group_size,
                 if (ts > 1) tail = std::max(tail, tail_bytes(ts, M, N, from) + 256);
             }
     }
-    if (!raw_applicable(M, K, group_size, quant) && option_value(MNQ_OPT_BF16_FP16_TILES) == 0)
+    if (!raw_applicable(M, K, group_size, quant) && !half_tiles && option_value(MNQ_OPT_BF16_FP16_TILES) == 0)
         return tail ? ((std::max(base, kCounterBytes) + 255) & ~size_t(255)) + tail : base;
     const int splits = base > kCounterBytes ? static_cast<int>((base - kCounterBytes) / (static_cast<size_t>(M) * N * 4)) : 1;
     return ((raw_region_offset(splits, M, N) + raw_region_bytes(M, K, true) + 255) & ~size_t(255)) + tail;

@@ -285,6 +285,16 @@ inline bool few_rows_small_layer(const MatmulArgs& a) { return a.N < 8192 && pac
 // Groups, or rows, of an odd number of 32s.
 inline bool odd_halves(int64_t K, int64_t group_size) { return K % 64 != 0 || (group_size < K && group_size % 64 != 0); }
 
+// Symmetric int4 with bf16 scales: a weight (q - 8) s has at most 8 + 3 significant bits (|q - 8| is 8 or at most 7), so
+// an fp16 tile holds it exactly once the row's scales are divided by a power of two; bf16 activations, divided by one per
+// token, fit fp16 exactly too.  Such calls take one fp16 tile per k-block (HalfTile in gemm_tcgen05.cu) where others with
+// bf16 activations and group-wise scales need two bf16 tiles, and lose nothing by it: what fp16 cannot hold lies 2^25
+// below a row's, or 2^29 below a token's, largest value, beyond the fp32 sums.
+inline bool exact_half_tiles(int64_t K, int64_t group_size, int32_t quant, int32_t act_dtype, int32_t scale_dtype, bool zeros)
+{
+    return quant == MNQ_INT4 && act_dtype == MNQ_BF16 && scale_dtype == MNQ_BF16 && !zeros && group_size < K && !odd_halves(K, group_size);
+}
+
 // Process-wide options (mnq_set_option); defined in api.cu.
 int64_t option_value(int option);
 
@@ -337,7 +347,8 @@ int read_device_status(unsigned int* out, bool clear);
 size_t gemv_stream_workspace_bytes(int64_t M, int64_t N, int64_t K, int32_t group_size, int32_t quant, bool* supported);
 size_t gemv_workspace_bytes(int64_t M, int64_t N, int64_t K, int32_t group_size, int32_t quant);
 bool gemm_supported(const MatmulArgs& a);
-size_t gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, int32_t group_size, int32_t quant);
+// half_tiles: with room for the fp16 copy of bf16 activations
+size_t gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, int32_t group_size, int32_t quant, bool half_tiles = false);
 size_t gemm_split_workspace_bytes(int64_t M, int64_t N, int64_t K, int32_t group_size);
 int launch_gemm(const MatmulArgs& a, const mnq_tuning* tuning);
 

@@ -58,6 +58,8 @@ def _load() -> ctypes.CDLL:
     L.mnq_version.argtypes = []
     L.mnq_workspace_bytes.restype = sz
     L.mnq_workspace_bytes.argtypes = [i64, i64, i64, i32, i32]
+    L.mnq_workspace_bytes_for.restype = sz
+    L.mnq_workspace_bytes_for.argtypes = [i64, i64, i64, i32, i32, i32, i32, i32]
     mm = [vp, vp, vp, vp, vp, i64, i64, i64, i64, i64, i32, i32, i32, i32, vp, sz, vp]
     L.mnq_dequant_matmul.restype = ctypes.c_int
     L.mnq_dequant_matmul.argtypes = mm
@@ -338,7 +340,7 @@ def dequant_matmul(activations, weights_packed, scales, zeros, group_size, quant
         with torch.cuda.device(dev):
             return dequant_matmul(x, weights_packed, s, z, g, quant_type, out=out, tuning=tuning)
     stream = torch.cuda.current_stream(dev).cuda_stream
-    nbytes = _lib.mnq_workspace_bytes(M, N, K, g, q)
+    nbytes = _lib.mnq_workspace_bytes_for(M, N, K, g, q, _DT[x.dtype], _DT[s.dtype], z is not None)
     ws = _workspace(dev, stream, nbytes)
     args = (x.data_ptr(), w.data_ptr(), s.data_ptr(), z.data_ptr() if z is not None else None,
             out.data_ptr(), M, N, K, lda, ldc, g, q, _DT[x.dtype], _DT[s.dtype],
@@ -426,7 +428,7 @@ def dequant_matmul_fused(activations, weights_packed, scales, zeros, group_size,
     ldr = (residual.stride(0) if M > 1 else max(N, 1)) if residual is not None else max(N, 1)
     with torch.cuda.device(dev):
         stream = torch.cuda.current_stream(dev).cuda_stream
-        ws = _workspace(dev, stream, _lib.mnq_workspace_bytes(M, N, K, g, q))
+        ws = _workspace(dev, stream, _lib.mnq_workspace_bytes_for(M, N, K, g, q, _DT[x.dtype], _DT[s.dtype], z is not None))
         _check(_lib.mnq_dequant_matmul_fused(
             x.data_ptr(), w.data_ptr(), s.data_ptr(), z.data_ptr() if z is not None else None, out.data_ptr(),
             M, N, K, lda, ldc, g, q, _DT[x.dtype], _DT[s.dtype], _DT[odt], EPILOGUES[epilogue],
@@ -664,7 +666,7 @@ def library_path() -> str:
 
 def exported_symbols() -> list[str]:
     """Entry points declared in include/mnq.h that this module binds."""
-    return ["mnq_status_name", "mnq_last_error", "mnq_version", "mnq_workspace_bytes",
+    return ["mnq_status_name", "mnq_last_error", "mnq_version", "mnq_workspace_bytes", "mnq_workspace_bytes_for",
             "mnq_dequant_matmul", "mnq_dequant_matmul_ex", "mnq_select_path", "mnq_dequantize",
             "mnq_dequantize_flat", "mnq_device_status", "mnq_dequant_matmul_gather", "mnq_host_workspace_bytes",
             "mnq_dequant_matmul_host", "mnq_dequant_matmul_swiglu", "mnq_select_path_ex", "mnq_set_option",
