@@ -463,7 +463,7 @@ template <> struct StageIO<__nv_bfloat16> {
 // T: the activation type (what bias and residual hold).  FINAL: the values stored are the
 // operator's result, so the epilogue is applied while they are staged; otherwise (a K split's
 // fp32 plane) they are stored as they are.
-// TOK: prepared activations (raw-integer tiles, HalfTile): the value of the tile's token c is acc * scale * f[c], with
+// TOK: prepared activations (raw-integer tiles, HalfTile): the value of the tile's token c is acc * (scale * f[c]), with
 // f the `tok` floats at shared address tok_at, and for raw-integer tiles (SUMS) - zterm * x[c], x the `tok` floats after
 // them.  (Read from global memory, two loads and a clamp for every element, they made the epilogue of 512 tokens x 128
 // rows last 35 us: [512, 4096] x [14336, 4096] int4 bf16 as one fp16 tile 86 us, from shared memory 55.)
@@ -496,7 +496,7 @@ __device__ __forceinline__ void epilogue_tile(uint32_t tmem_base, int quad, int 
                     const uint32_t fw[4] = {f.x, f.y, f.z, f.w}, xw[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {
-                        float val = __uint_as_float(v[i + k]) * scale * __uint_as_float(fw[k]);
+                        float val = __uint_as_float(v[i + k]) * (scale * __uint_as_float(fw[k]));   // (a power of two: exact; either alone may be out of range)
                         if (SUMS) val = fmaf(-zterm, __uint_as_float(xw[k]), val);
                         v[i + k] = __float_as_uint(val);
                     }
@@ -836,7 +836,7 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap
                 mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
                 // E = floor(log2(mx)) from the exponent field (zero, subnormal, inf or nan rows: E = 0)
                 const int ex = static_cast<int>((__float_as_uint(mx) >> 23) & 0xFFu);
-                const int E = (ex == 0 || ex == 255) ? 0 : max(-100, min(100, ex - 127));
+                const int E = (ex == 0 || ex == 255) ? 0 : max(-126, min(126, ex - 127));
                 down = __int_as_float(static_cast<uint32_t>(127 - E) << 23);
                 if (hp == 0) row_up[rr] = __int_as_float(static_cast<uint32_t>(127 + E) << 23);
             }
@@ -1173,8 +1173,8 @@ __global__ void __launch_bounds__(256) prep_activations_kernel(const T* __restri
 #pragma unroll
         for (int w = 0; w < 8; ++w) mx = max(mx, warp_max[w]);
         const int E = static_cast<int>(mx >> 7);           // biased bf16 exponent of the maximum
-        int sh = (E == 0) ? 0 : (E - 127) - 14;
-        sh = max(-100, min(100, sh));
+        // (a maximum of 2^127 still lands inside fp16; 2^120 brings a subnormal maximum well above fp16's smallest)
+        const int sh = max(-120, min(120, E == 0 ? -120 : (E - 127) - 14));
         down = __int_as_float((127 - sh) << 23);
         up = __int_as_float((127 + sh) << 23);
     }

@@ -44,6 +44,24 @@ def test_exact_half_tiles(M, N, K, g, spread):
     assert torch.equal(out, out32.to(torch.bfloat16))
 
 
+@pytest.mark.parametrize("x_exp,s_exp", [(120, -20), (-120, 20), (-128, 100), (30, -110), (-110, 118)])
+def test_the_ends_of_bf16s_range(x_exp, s_exp):
+    """Activations and scales near bf16's largest and smallest values (2^-128: subnormal): the powers of two that bring them into fp16 reach."""
+    import metal_native
+    import mnq_workloads as workloads
+    C = metal_native._C
+    L = workloads.make_layer("t", 72, 512, 256, quant_type="int4", group_size=128, act_dtype=torch.bfloat16,
+                             scale_dtype=torch.bfloat16, asymmetric=False, seed=9)
+    L.x = (L.x.double() * 2.0 ** x_exp).to(torch.bfloat16)
+    L.scales = (L.scales.double() * 2.0 ** s_exp).to(torch.bfloat16)
+    d = L.to("cuda")
+    out32 = C.dequant_matmul_fused(*d.args(), out_dtype=torch.float32)
+    W = metal_native.dequantize(d.wq, d.scales, None, 128, "int4", torch.float32).double()
+    ref = d.x.double() @ W.t()
+    assert bool(torch.isfinite(out32).all())
+    assert float((out32.double() - ref).norm() / ref.norm()) < 2e-6
+
+
 def test_little_workspace_takes_the_two_tiles():
     """A caller that brings what mnq_workspace_bytes names gets the kernel that needs no more."""
     import metal_native
