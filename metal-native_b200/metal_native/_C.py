@@ -340,7 +340,10 @@ def dequant_matmul(activations, weights_packed, scales, zeros, group_size, quant
         with torch.cuda.device(dev):
             return dequant_matmul(x, weights_packed, s, z, g, quant_type, out=out, tuning=tuning)
     stream = torch.cuda.current_stream(dev).cuda_stream
-    nbytes = _lib.mnq_workspace_bytes_for(M, N, K, g, q, _DT[x.dtype], _DT[s.dtype], z is not None)
+    if M <= 32:   # (the types make no difference there, and a decode call is short)
+        nbytes = _lib.mnq_workspace_bytes(M, N, K, g, q)
+    else:
+        nbytes = _lib.mnq_workspace_bytes_for(M, N, K, g, q, _DT[x.dtype], _DT[s.dtype], z is not None)
     ws = _workspace(dev, stream, nbytes)
     args = (x.data_ptr(), w.data_ptr(), s.data_ptr(), z.data_ptr() if z is not None else None,
             out.data_ptr(), M, N, K, lda, ldc, g, q, _DT[x.dtype], _DT[s.dtype],
